@@ -46,6 +46,9 @@ def _torch() -> Any:
     return torch
 
 
+_UPLOAD_ALIGN = 128  # int32 words: 512 bytes
+
+
 @dataclass(slots=True, frozen=True)
 class PagedKVCache:
     key_pages: Any
@@ -97,6 +100,8 @@ class ClusteredPageDecodePlan:
 
     def device_tensors(self, device: Any) -> dict[str, Any]:
         """The six descriptor arrays as int32 tensors on `device`, uploaded once per device."""
+        import numpy as np
+
         torch = _torch()
         key = str(device)
         if key not in self._device_cache:
@@ -108,9 +113,15 @@ class ClusteredPageDecodePlan:
                 "request_run_offsets": self.request_run_offsets_cpu,
                 "seq_lens": self.seq_lens_cpu,
             }
-            self._device_cache[key] = {
-                name: tensor.to(device=device, dtype=torch.int32) for name, tensor in host.items()
-            }
+            # one buffer and one copy for the six; every array starts where an allocation of its own would
+            parts, sizes = [], []
+            for tensor in host.values():
+                values = tensor.to(device="cpu", dtype=torch.int32).numpy()
+                gap = -values.size % _UPLOAD_ALIGN
+                parts += [values, np.zeros(gap, dtype=np.int32)]
+                sizes += [values.size, gap]
+            uploaded = torch.from_numpy(np.concatenate(parts)).to(device=device).split(sizes)
+            self._device_cache[key] = dict(zip(host, uploaded[::2]))
         return self._device_cache[key]
 
 
@@ -468,36 +479,36 @@ def plan_clustered_page_decode(
         "clustered" if group_size > 8 or max_pages > direct_page_threshold else "direct")
 
     table = table_cpu.numpy()
-    cache_key = (lens.tobytes(), table.tobytes(), table.shape, num_q_heads, num_kv_heads, head_dim, page_size,
-                 layout, group_tile, chosen_cluster, direct_page_threshold, pdl_page_threshold)
-    if use_cache and cache_key in _PLAN_CACHE:
-        return _PLAN_CACHE[cache_key]
+    if use_cache:
+        cache_key = (lens.tobytes(), table.tobytes(), table.shape, num_q_heads, num_kv_heads, head_dim, page_size,
+                     layout, group_tile, chosen_cluster, direct_page_threshold, pdl_page_threshold)
+        if cache_key in _PLAN_CACHE:
+            return _PLAN_CACHE[cache_key]
 
-    bases: list[np.ndarray] = []
-    counts: list[np.ndarray] = []
-    starts: list[np.ndarray] = []
-    lasts: list[np.ndarray] = []
-    offsets = [0]
-    for request in range(batch):
-        n = int(pages[request])
-        if n > 0:
-            row = table[request, :n].astype(np.int64)
-            # a new run begins wherever a page does not follow its predecessor physically
-            begin = np.concatenate(([0], np.flatnonzero(np.diff(row) != 1) + 1))
-            length = np.diff(np.concatenate((begin, [n])))
-            last = np.full(begin.shape, page_size, dtype=np.int64)
-            last[-1] = (int(lens[request]) - 1) % page_size + 1
-            bases.append(row[begin])
-            counts.append(length)
-            starts.append(begin)
-            lasts.append(last)
-            offsets.append(offsets[-1] + int(begin.size))
-        else:
-            offsets.append(offsets[-1])
+    # All requests at once (a serving step plans anew for every token, and a loop of a few numpy calls
+    # per request took most of the step): a run begins wherever a page does not follow its
+    # predecessor physically, and ends where the next one begins or the request's pages end.
+    if max_pages > 0 and table.shape[1] == 0:
+        raise IndexError("page_table has no columns")
+    width = int(table.shape[1])
+    begins = np.ones(table.shape, dtype=bool)
+    np.not_equal(table[:, 1:], table[:, :-1] + np.int64(1), out=begins[:, 1:])
+    begins &= np.arange(width) < pages[:, None]
+    runs = begins.sum(axis=1)
+    offsets = np.zeros(batch + 1, dtype=np.int64)
+    np.cumsum(runs, out=offsets[1:])
+    # request by request, pages in order
+    starts = np.flatnonzero(begins) - np.repeat(np.arange(batch) * width, runs)
+    owners = np.flatnonzero(runs)
+    final = offsets[1:][owners] - 1  # the last run of each request that has any
+    ends = np.empty_like(starts)
+    ends[:-1] = starts[1:]
+    ends[final] = pages[owners]
+    lasts = np.full(starts.shape, page_size, dtype=np.int64)
+    lasts[final] = (lens[owners] - 1) % page_size + 1
 
-    def as_tensor(parts: list[np.ndarray]) -> Any:
-        joined = np.concatenate(parts) if parts else np.empty((0,), dtype=np.int64)
-        return torch.from_numpy(joined.astype(np.int32))
+    def as_tensor(values: np.ndarray) -> Any:
+        return torch.from_numpy(values.astype(np.int32))
 
     plan = ClusteredPageDecodePlan(
         batch=batch,
@@ -513,11 +524,11 @@ def plan_clustered_page_decode(
         direct_page_threshold=direct_page_threshold,
         pdl_page_threshold=pdl_page_threshold,
         launch_mode=launch_mode,
-        run_base_pages_cpu=as_tensor(bases),
-        run_page_counts_cpu=as_tensor(counts),
+        run_base_pages_cpu=as_tensor(table[begins]),
+        run_page_counts_cpu=as_tensor(ends - starts),
         run_logical_starts_cpu=as_tensor(starts),
         run_last_page_lens_cpu=as_tensor(lasts),
-        request_run_offsets_cpu=torch.tensor(offsets, dtype=torch.int32),
+        request_run_offsets_cpu=as_tensor(offsets),
         seq_lens_cpu=seq_lens_cpu,
     )
     if use_cache:

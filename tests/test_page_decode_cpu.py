@@ -229,3 +229,39 @@ def test_native_module_exposes_the_reference_name_and_keywords() -> None:
                     "rope_theta", "stream_ptr"):
         assert keyword in doc
     assert KV_IDS == ops.KV_FORMAT_IDS
+
+
+@pytest.mark.parametrize("seed", range(8))
+def test_plan_runs_equal_a_page_by_page_walk(seed: int) -> None:
+    """Runs of a batch planned at once: empty and ragged requests, pages in any order (neighbours,
+    repeats, -1 behind a request's end), either integer type, a table that is not contiguous."""
+    rng = torch.Generator().manual_seed(seed)
+    batch, width, page = 7, 9, (16, 32)[seed % 2]
+    lens = torch.randint(-2, width * page + 1, (batch,), generator=rng)
+    lens[seed % batch] = 0
+    table = torch.randint(0, 4, (width, batch), generator=rng).T + torch.arange(width) * (seed % 3 != 0)
+    table[:, -1] = -1
+    lens = torch.minimum(lens, torch.tensor((width - 1) * page))
+    if seed % 2:
+        table, lens = table.to(torch.int32), lens.to(torch.int32)
+    plan = ops.plan_clustered_page_decode(
+        page_table=table, seq_lens=lens, num_q_heads=4, num_kv_heads=2, head_dim=64, page_size=page,
+        kv_layout="bf16_kv", use_cache=False)
+    runs, offsets = [], [0]
+    for request in range(batch):
+        length = int(lens[request])
+        pages = max(0, -(-length // page))
+        for i in range(pages):
+            if i and int(table[request, i]) == int(table[request, i - 1]) + 1:
+                runs[-1][1] += 1
+            else:
+                runs.append([int(table[request, i]), 1, i, page])
+        if pages:
+            runs[-1][3] = (length - 1) % page + 1
+        offsets.append(len(runs))
+    device = plan.device_tensors("cpu")
+    names = ("run_base_pages", "run_page_counts", "run_logical_starts", "run_last_page_lens")
+    assert [device[name].tolist() for name in names] == [[run[i] for run in runs] for i in range(4)]
+    assert device["request_run_offsets"].tolist() == offsets
+    assert device["seq_lens"].tolist() == lens.tolist()
+    assert all(tensor.dtype == torch.int32 for tensor in device.values())
