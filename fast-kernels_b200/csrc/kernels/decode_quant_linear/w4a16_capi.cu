@@ -6,6 +6,7 @@
 #include <cublasLt.h>
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -22,6 +23,7 @@
 #include "w4a16_gemv_chain.cuh"
 #include "w4a16_gemv_wmma.cuh"
 #include "w4a16_launch.h"
+#include "w4a16_tile_plan.cuh"
 #include "w4a16_umma_plan.cuh"
 #include "w4a16_prep.cuh"
 
@@ -221,6 +223,7 @@ struct Tuning {
   int wmma = 0;            // FK_W4A16_WMMA: batches 1-2 on the warp-level mma.sync form
   int umma_min_batch = -1; // FK_W4A16_UMMA_MIN_BATCH: smallest batch for the pipelined tcgen05 kernel
                            // (-1 = built-in default, 0 = never)
+  int tile_min_batch = -1; // FK_W4A16_TILE_MIN_BATCH: smallest batch for the tile kernel (-1 = rule, 0 = never)
   int peer_wait_ms = 2000; // FK_W4A16_PEER_WAIT_MS: how long a multi-GPU call waits for the other GPUs
   int cluster = 1;         // FK_W4A16_CLUSTER: 0 keeps layers with few tiles off the cluster kernel
 };
@@ -234,6 +237,8 @@ Tuning& tuning() {
     g_tuning.wmma = env_int("FK_W4A16_WMMA");
     const char* text = std::getenv("FK_W4A16_UMMA_MIN_BATCH");
     g_tuning.umma_min_batch = text == nullptr ? -1 : std::atoi(text);
+    text = std::getenv("FK_W4A16_TILE_MIN_BATCH");
+    g_tuning.tile_min_batch = text == nullptr ? -1 : std::atoi(text);
     if (env_int("FK_W4A16_PEER_WAIT_MS") > 0) {
       g_tuning.peer_wait_ms = env_int("FK_W4A16_PEER_WAIT_MS");
     }
@@ -259,6 +264,8 @@ struct Plan {
   bool tensor_cores = false;  // batch > 4: the MMA kernel, rows in tiles of 8 or 16
   bool wmma = false;          // batch <= 2: the stream kernel with its inner product on mma.sync
   bool umma = false;          // the pipelined tcgen05 kernel: one run per CTA, rows in {1,2,4,8,16}
+  bool tile = false;          // batches on tcgen05, m_tile rows a pass (w4a16_gemm_tile.cuh)
+  uint32_t blocks = 0;        // its steps per unit
   size_t staged_bytes = 0;    // its pre-staged activations, behind the scratch slots
 };
 
@@ -486,6 +493,75 @@ Plan make_umma_plan(int batch, int n, int k, int group_size, int sm_count, int m
   plan.smem_bytes = plan.smem_bytes < floor_bytes ? floor_bytes : plan.smem_bytes;
   plan.scratch_bytes = static_cast<size_t>(plan.row_tiles) * plan.grid_x * 2 *
                        (plan.m_tile * kTileCols) * sizeof(float);
+  return plan;
+}
+
+// Which problems take the tile kernel by default (FK_W4A16_TILE_MIN_BATCH overrides the rule with a
+// smallest batch; 0 there means "never"). Above 8 rows the mma.sync kernel reads the layer once per
+// 16 rows (28672 x 8192, bf16: 58 / 112 / 221 / 862 us at 16 / 32 / 64 / 256 rows, against 51 / 57 /
+// 68 / 204 here). Its passes run side by side where the layer is too small to fill the chip with
+// one, which is worth more above 64 rows (512 x 1024, 128 rows: 18 us against 28; 1024 x 4096: 34
+// against 39), and no longer at 2048 x 4096 (45 against 39). At 8 rows and fewer the mma.sync
+// kernel keeps its lead (28672 x 8192: 34 us against 50).
+bool tile_wanted(int batch, int n, int k) {
+  if (umma_forced() >= 0) {
+    return false;
+  }
+  const int min_batch = tuning().tile_min_batch;
+  if (min_batch >= 0) {
+    return min_batch > 0 && batch >= min_batch;
+  }
+  return batch > 8 && (batch <= 64 || static_cast<long long>(n) * k >= 6ll << 20);
+}
+
+// Plan of the tile kernel; stages = 0 where it does not apply.
+Plan make_tile_plan(int batch, int n, int k, int group_size, int sm_count, int max_smem,
+                    const LaunchConfig& cfg) {
+  Plan plan;
+  plan.tile = true;
+  const long long tiles = n / kTileCols;
+  plan.total_packets = static_cast<uint32_t>(tiles * (k / group_size));
+  plan.row_tiles = (batch + kTileMaxRows - 1) / kTileMaxRows;
+  plan.m_tile = (((batch + plan.row_tiles - 1) / plan.row_tiles) + 15) & ~15;
+  plan.blocks = static_cast<uint32_t>((k + kTileK - 1) / kTileK);
+  const long long units = ((tiles + kTilePair - 1) / kTilePair) * plan.row_tiles;
+  const long long steps = units * plan.blocks;
+  // a ticket per unit, tile and warp; 32-bit step numbers
+  if (units * kTilePair * 4 > kTicketCapacity - 2 || steps > INT_MAX) {
+    return plan;
+  }
+  // Few units: a whole number of CTAs for each, so that no CTA has to hand in parts of two, and no
+  // more than pay. One more CTA shortens a unit's steps / c by a share and costs whoever finishes the
+  // unit one more read of its rows; the sum was least near c^2 = 5/4 steps (1024 x 28672, 224 steps,
+  // 16 rows: 30.1 / 28.6 / 30.3 / 35.6 us with 12 / 16 / 24 / 37 CTAs a unit; 4096 x 4096, 32 steps,
+  // 128 rows: 43 us with 4, 50 with 8). With more units than that leaves CTAs for, every SM takes an
+  // equal share of the steps.
+  long long ctas = cfg.ctas > 0 ? cfg.ctas : sm_count;
+  if (cfg.ctas <= 0) {
+    long long share = sm_count / units;
+    while (share > 1 && (share - 1) * (share - 1) * 4 >= 5ll * plan.blocks) {
+      --share;
+    }
+    if (share >= 2 && (share < sm_count / units || share * units * 4 >= 3ll * sm_count || share >= 4)) {
+      ctas = share * units;
+    }
+  }
+  ctas = ctas > 256 ? 256 : ctas;
+  ctas = ctas > steps ? steps : ctas;
+  plan.grid_x = static_cast<int>(ctas);
+  plan.active_warps = plan.grid_x;
+  plan.warps = kTileThreads / 32;
+  const int stage = tile_stage_bytes(group_size, plan.m_tile);
+  const int fit = (max_smem - kTileBarrierBytes) / stage;
+  int wanted = cfg.stages > 0 ? cfg.stages : kTileMaxStages;
+  wanted = wanted > kTileMaxStages ? kTileMaxStages : wanted;
+  plan.stages = fit < wanted ? fit : wanted;
+  plan.smem_bytes = kTileBarrierBytes + (static_cast<size_t>(plan.stages) * stage);
+  // one CTA per SM: each allocates all of the SM's tensor memory
+  const size_t floor_bytes = (static_cast<size_t>(max_smem) / 2) + 1024;
+  plan.smem_bytes = plan.smem_bytes < floor_bytes ? floor_bytes : plan.smem_bytes;
+  plan.scratch_bytes = static_cast<size_t>(plan.grid_x) * 2 * kTilePair * plan.m_tile * kTileCols * sizeof(float);
+  plan.staged_bytes = static_cast<size_t>(plan.row_tiles) * plan.blocks * tile_block_bytes(group_size, plan.m_tile);
   return plan;
 }
 
@@ -741,6 +817,8 @@ int fk_w4a16_set_tuning(const char* name, int value) {
     t.wmma = value;
   } else if (key == "umma_min_batch") {
     t.umma_min_batch = value;
+  } else if (key == "tile_min_batch") {
+    t.tile_min_batch = value;
   } else if (key == "cluster") {
     t.cluster = value != 0 ? 1 : 0;
   } else if (key == "peer_wait_ms") {
@@ -826,6 +904,11 @@ size_t fk_w4a16_workspace_bytes(int batch, int n, int k, int group_size) {
       make_umma_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
   size_t need = workspace_bytes_for(plan);
   need = need > workspace_bytes_for(umma_plan) ? need : workspace_bytes_for(umma_plan);
+  const Plan tile_plan =
+      make_tile_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
+  if (tile_wanted(batch, n, k) && tile_plan.stages >= 2) {
+    need = need > workspace_bytes_for(tile_plan) ? need : workspace_bytes_for(tile_plan);
+  }
   return need;
 }
 
@@ -839,11 +922,16 @@ int fk_w4a16_describe_plan(int batch, int n, int k, int group_size, int dtype, c
   DeviceInfo* info = nullptr;
   FK_TRY(device_info(&info));
   const bool use_umma = umma_wanted(batch, n, k, group_size);
+  const Plan tile_plan =
+      make_tile_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
   const Plan plan =
       use_umma ? make_umma_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config())
-               : make_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config(),
+      : tile_wanted(batch, n, k) && tile_plan.stages >= 2
+          ? tile_plan
+          : make_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config(),
                       /*allow_cluster=*/true, /*cuda_cores_only=*/false);
   const char* kernel = plan.umma            ? "w4a16_gemm_umma_kernel"
+                       : plan.tile          ? "w4a16_gemm_tile_kernel"
                        : plan.tensor_cores  ? "w4a16_gemm_mma_kernel"
                        : plan.wmma          ? "w4a16_gemv_wmma_kernel"
                        : plan.cluster_size > 1 ? "w4a16_gemv_cluster_kernel"
@@ -977,9 +1065,21 @@ int gemv_impl(const fk_w4a16_gemv_args* args, bool with_exchange_area, bool smal
   }
   // The fused RMSNorm lives in the CUDA-core kernels (stream and cluster).
   const bool use_umma = !normalise && !small_batch_on_cuda_cores && umma_wanted(batch, n, k, group_size);
+  // The tile kernel stores plain outputs (with a residual, placed or in fp32): the gated epilogue and
+  // everything that involves other GPUs stay with the packet-stream kernels, and so does a call whose
+  // workspace is large enough for those only.
+  const Plan tile_plan =
+      make_tile_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
+  const bool use_tile = !use_umma && !normalise && !small_batch_on_cuda_cores && with_exchange_area && !gated &&
+                        args->num_peers == 0 && args->local_signal == nullptr && args->reduce_slots == 0 &&
+                        args->ll_epoch == 0 && args->ll_epoch_counter == nullptr &&
+                        tile_wanted(batch, n, k) && tile_plan.stages >= 2 &&
+                        args->workspace_bytes >= workspace_bytes_for(tile_plan, header_bytes);
   const Plan plan =
       use_umma
           ? make_umma_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config())
+      : use_tile
+          ? tile_plan
           : make_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config(),
                       /*allow_cluster=*/true,
                       /*cuda_cores_only=*/normalise || small_batch_on_cuda_cores);
@@ -994,7 +1094,8 @@ int gemv_impl(const fk_w4a16_gemv_args* args, bool with_exchange_area, bool smal
     return fail(FK_W4A16_ERR_INVALID_ARGUMENT, oss.str());
   }
   const int num_tiles = n / kTileCols;
-  if (static_cast<long long>(plan.row_tiles) * num_tiles > kTicketCapacity - 2) {
+  const int ticket_rows = use_tile ? stream_plan.row_tiles : plan.row_tiles;  // one limit, whichever kernel runs
+  if (static_cast<long long>(ticket_rows) * num_tiles > kTicketCapacity - 2) {
     return fail(FK_W4A16_ERR_INVALID_ARGUMENT, "n * batch exceeds the ticket area of a workspace");
   }
 
@@ -1016,7 +1117,7 @@ int gemv_impl(const fk_w4a16_gemv_args* args, bool with_exchange_area, bool smal
   const size_t gated_bytes =
       gated ? static_cast<size_t>(batch) * (n / 2) * sizeof(unsigned long long) : 0;
   const bool wants_exchange =
-      with_exchange_area && !plan.tensor_cores && plan.cluster_size == 1 && plan.m_tile <= 4;
+      with_exchange_area && !plan.tensor_cores && !plan.tile && plan.cluster_size == 1 && plan.m_tile <= 4;
   // (the pipelined tcgen05 kernel finishes split tiles like the packet-stream kernel does)
   if (!wants_exchange || exchange_bytes + gated_bytes > kExchangeBytes) {
     exchange_bytes = 0;  // split tiles take the ticket finish; the area is the epilogue's alone
@@ -1093,6 +1194,28 @@ int gemv_impl(const fk_w4a16_gemv_args* args, bool with_exchange_area, bool smal
     launch.programmatic = pdl_enabled();
     launch.stream = s;
     FK_TRY_CUDA(launch_umma_kernel(params, launch));
+    return FK_W4A16_OK;
+  }
+  if (plan.tile) {
+    TileLaunch launch{};
+    launch.bf16 = args->dtype == FK_W4A16_DTYPE_BF16;
+    launch.rows = plan.m_tile;
+    launch.row_tiles = plan.row_tiles;
+    launch.blocks = plan.blocks;
+    launch.total_steps = static_cast<uint32_t>((num_tiles + kTilePair - 1) / kTilePair) *
+                         static_cast<uint32_t>(plan.row_tiles) * plan.blocks;
+    launch.ctas = plan.grid_x;
+    launch.stages = plan.stages;
+    launch.smem_bytes = plan.smem_bytes;
+    launch.max_smem = max_smem;
+    launch.staged = static_cast<uint8_t*>(args->workspace) + header_bytes +
+                    ((plan.scratch_bytes + 255) & ~size_t{255});
+    launch.slots = params.scratch;
+    launch.programmatic = pdl_enabled();
+    launch.stream = s;
+    FK_TRY_CUDA(group_size == 32   ? launch_tile_kernel<32>(params, launch)
+                : group_size == 64 ? launch_tile_kernel<64>(params, launch)
+                                   : launch_tile_kernel<128>(params, launch));
     return FK_W4A16_OK;
   }
   if (plan.tensor_cores) {

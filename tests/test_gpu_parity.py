@@ -664,6 +664,7 @@ def _gemv_ex(lib, act, packets, out, shape, code, *, f32=0, residual=None):
         (4096, 4096, 1, "bf16", 0),            # cluster kernel
         (28672, 4096, 2, "bf16", 0),           # pair-exchange finish
         (128 * 6, 128 * 5, 8, "bf16", 0),      # mma.sync kernel
+        (128 * 5, 128 * 9, 24, "bf16", 0),     # tile kernel
         (128 * 6, 128 * 5, 2, "bf16", 1),      # tcgen05 kernel
     ],
 )
@@ -831,6 +832,32 @@ def test_gemm_tensor_core_batches(group: int, batch: int, dtype: str) -> None:
     shape = LayerShape("t", 128 * 5, group * 9, group_size=group, batch=batch, dtype=dtype,
                        zero_point=None, scale_range=(0.001, 0.05))
     _check_gemv(make_problem(shape, seed=13 * group + batch), shape, oracle.dtype_code(dtype))
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize(("batch", "tiles", "features"), [
+    (5, 1, 128),      # one step in all
+    (17, 5, 1152),    # 32 rows a pass, 17 of them real; an odd number of tiles; units shared by CTAs
+    (33, 2, 1088),    # K ends inside a step for groups of 32 and 64
+    (64, 301, 256),   # more units than CTAs: runs that begin and end inside a unit, whole units between
+    (65, 4, 1152), (112, 3, 1088), (128, 7, 640),
+    (129, 5, 1152),   # two row tiles of 80 rows, the second with 49
+    (256, 6, 1024), (300, 3, 384),
+])
+def test_gemm_tile_batches(group: int, dtype: str, batch: int, tiles: int, features: int) -> None:
+    """The tcgen05 tile kernel (tuning knob "tile_min_batch" sends every batch to it): up to 128 rows
+    a pass in multiples of 16, two weight tiles and 128 features a step."""
+    lib = capi.load_library()
+    features = features // group * group
+    shape = LayerShape("t", 128 * tiles, features, group_size=group, batch=batch, dtype=dtype,
+                       zero_point=None, scale_range=(0.001, 0.05))
+    capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", 1))
+    try:
+        assert "gemm_tile" in capi.describe_plan(batch, shape.n, shape.k, group, oracle.dtype_code(dtype))
+        _check_gemv(make_problem(shape, seed=17 * group + batch), shape, oracle.dtype_code(dtype))
+    finally:
+        capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
 
 
 @pytest.mark.parametrize(("n", "k", "batch"), [(4096, 4096, 8), (28672, 8192, 16), (4096, 14336, 8)])
