@@ -52,7 +52,7 @@ def build_library(force: bool = False) -> Path:
     """libfk_w4a16.so: every CUDA kernel plus the extern "C" entry points of include/fk_w4a16.h."""
     kernel_dir = CSRC / "kernels" / "decode_quant_linear"
     sources = sorted(kernel_dir.glob("*.cu"))
-    deps = sources + sorted(kernel_dir.glob("*.cuh")) + sorted(kernel_dir.glob("*.h")) + [REPO / "include" / "fk_w4a16.h"]
+    deps = sources + sorted(kernel_dir.glob("*.cuh")) + sorted(kernel_dir.glob("*.h")) + sorted(kernel_dir.glob("*.inc")) + [REPO / "include" / "fk_w4a16.h"]
     target = LIB_DIR / "libfk_w4a16.so"
     if not force and _newer(target, deps):
         return target
