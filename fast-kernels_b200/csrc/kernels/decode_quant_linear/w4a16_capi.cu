@@ -1669,12 +1669,13 @@ int fk_w4a16_dequant_packets(const void* packets, void* weight, int n, int k, in
   FK_TRY(check_pointer(weight, "weight", 16));
   DeviceInfo* info = nullptr;
   FK_TRY(device_info(&info));
-  const long long total_words = static_cast<long long>(n) * (k / 8);
-  const int grid = grid_for(total_words, 256, info->sm_count);
+  const long long total_packets = static_cast<long long>(n / kTileCols) * (k / group_size);
+  const long long cap = static_cast<long long>(info->sm_count) * 8;  // resident CTAs of 256 threads
+  const int grid = static_cast<int>(total_packets < cap ? total_packets : cap);
   auto* s = static_cast<cudaStream_t>(stream);
   const int rc = dispatch(group_size, 1, dtype, [&](auto g, auto, auto e) {
     dequant_packets_kernel<decltype(g)::value, decltype(e)><<<grid, 256, 0, s>>>(
-        static_cast<const uint8_t*>(packets), static_cast<uint16_t*>(weight), total_words, k,
+        static_cast<const uint8_t*>(packets), static_cast<uint16_t*>(weight), total_packets, k,
         k / group_size);
     return FK_W4A16_OK;
   });
