@@ -565,6 +565,14 @@ Plan make_tile_plan(int batch, int n, int k, int group_size, int sm_count, int m
   return plan;
 }
 
+// The plan where the rule wants the kernel, else (and where it cannot run) one with fewer than two
+// stages: small batches, whose calls are bound by host work, pay for the rule alone.
+Plan tile_plan_if_wanted(int batch, int n, int k, int group_size, const DeviceInfo& info) {
+  return tile_wanted(batch, n, k)
+             ? make_tile_plan(batch, n, k, group_size, info.sm_count, info.max_smem_optin, launch_config())
+             : Plan{};
+}
+
 size_t workspace_bytes_for(const Plan& plan, size_t header_bytes = kHeaderBytes) {
   return header_bytes + ((plan.scratch_bytes + 255) & ~size_t{255}) +
          ((plan.staged_bytes + 255) & ~size_t{255});
@@ -904,9 +912,8 @@ size_t fk_w4a16_workspace_bytes(int batch, int n, int k, int group_size) {
       make_umma_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
   size_t need = workspace_bytes_for(plan);
   need = need > workspace_bytes_for(umma_plan) ? need : workspace_bytes_for(umma_plan);
-  const Plan tile_plan =
-      make_tile_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
-  if (tile_wanted(batch, n, k) && tile_plan.stages >= 2) {
+  const Plan tile_plan = tile_plan_if_wanted(batch, n, k, group_size, *info);
+  if (tile_plan.stages >= 2) {
     need = need > workspace_bytes_for(tile_plan) ? need : workspace_bytes_for(tile_plan);
   }
   return need;
@@ -922,11 +929,10 @@ int fk_w4a16_describe_plan(int batch, int n, int k, int group_size, int dtype, c
   DeviceInfo* info = nullptr;
   FK_TRY(device_info(&info));
   const bool use_umma = umma_wanted(batch, n, k, group_size);
-  const Plan tile_plan =
-      make_tile_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
+  const Plan tile_plan = tile_plan_if_wanted(batch, n, k, group_size, *info);
   const Plan plan =
       use_umma ? make_umma_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config())
-      : tile_wanted(batch, n, k) && tile_plan.stages >= 2
+      : tile_plan.stages >= 2
           ? tile_plan
           : make_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config(),
                       /*allow_cluster=*/true, /*cuda_cores_only=*/false);
@@ -1068,12 +1074,11 @@ int gemv_impl(const fk_w4a16_gemv_args* args, bool with_exchange_area, bool smal
   // The tile kernel stores plain outputs (with a residual, placed or in fp32): the gated epilogue and
   // everything that involves other GPUs stay with the packet-stream kernels, and so does a call whose
   // workspace is large enough for those only.
-  const Plan tile_plan =
-      make_tile_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
+  const Plan tile_plan = tile_plan_if_wanted(batch, n, k, group_size, *info);
   const bool use_tile = !use_umma && !normalise && !small_batch_on_cuda_cores && with_exchange_area && !gated &&
                         args->num_peers == 0 && args->local_signal == nullptr && args->reduce_slots == 0 &&
                         args->ll_epoch == 0 && args->ll_epoch_counter == nullptr &&
-                        tile_wanted(batch, n, k) && tile_plan.stages >= 2 &&
+                        tile_plan.stages >= 2 &&
                         args->workspace_bytes >= workspace_bytes_for(tile_plan, header_bytes);
   const Plan plan =
       use_umma

@@ -100,11 +100,11 @@ class ClusteredPageDecodePlan:
 
     def device_tensors(self, device: Any) -> dict[str, Any]:
         """The six descriptor arrays as int32 tensors on `device`, uploaded once per device."""
-        import numpy as np
-
         torch = _torch()
         key = str(device)
         if key not in self._device_cache:
+            import numpy as np
+
             host = {
                 "run_base_pages": self.run_base_pages_cpu,
                 "run_page_counts": self.run_page_counts_cpu,
