@@ -490,21 +490,22 @@ def plan_clustered_page_decode(
     # predecessor physically, and ends where the next one begins or the request's pages end.
     if max_pages > 0 and table.shape[1] == 0:
         raise IndexError("page_table has no columns")
-    width = int(table.shape[1])
+    table = table[:, :max(max_pages, 0)]  # a serving table is as wide as the longest context allowed
     begins = np.ones(table.shape, dtype=bool)
     np.not_equal(table[:, 1:], table[:, :-1] + np.int64(1), out=begins[:, 1:])
-    begins &= np.arange(width) < pages[:, None]
-    runs = begins.sum(axis=1)
-    offsets = np.zeros(batch + 1, dtype=np.int64)
-    np.cumsum(runs, out=offsets[1:])
-    # request by request, pages in order
-    starts = np.flatnonzero(begins) - np.repeat(np.arange(batch) * width, runs)
-    owners = np.flatnonzero(runs)
-    final = offsets[1:][owners] - 1  # the last run of each request that has any
-    ends = np.empty_like(starts)
-    ends[:-1] = starts[1:]
+    if batch > 1:  # a single request uses every column that is left
+        begins &= np.arange(table.shape[1]) < pages[:, None]
+    firsts = np.arange(batch + 1) * table.shape[1]  # index of each request's first page
+    starts = begins.ravel().nonzero()[0]  # request by request, pages in order
+    offsets = starts.searchsorted(firsts)
+    if batch > 1:
+        starts -= firsts[:-1].repeat(offsets[1:] - offsets[:-1])
+    # the last run of a request ends with the request's pages, every other one where the next begins
+    owners = (pages > 0).nonzero()[0]
+    final = offsets[owners + 1] - 1
+    ends = np.append(starts[1:], 0)
     ends[final] = pages[owners]
-    lasts = np.full(starts.shape, page_size, dtype=np.int64)
+    lasts = np.full(starts.shape, page_size)
     lasts[final] = (lens[owners] - 1) % page_size + 1
 
     def as_tensor(values: np.ndarray) -> Any:

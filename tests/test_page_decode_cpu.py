@@ -7,6 +7,7 @@ from __future__ import annotations
 import ctypes
 import importlib
 import re
+import tracemalloc
 from pathlib import Path
 
 import numpy as np
@@ -265,3 +266,37 @@ def test_plan_runs_equal_a_page_by_page_walk(seed: int) -> None:
     assert device["request_run_offsets"].tolist() == offsets
     assert device["seq_lens"].tolist() == lens.tolist()
     assert all(tensor.dtype == torch.int32 for tensor in device.values())
+
+
+def test_plan_work_follows_the_pages_in_use_not_the_table_width() -> None:
+    """Serving tables are as wide as the longest context the model takes. Planning over one is the
+    same plan, and allocates no array of the table's size (numpy reports its buffers to tracemalloc)."""
+    batch, used, width = 4, 6, 1 << 18
+    table = torch.full((batch, width), -1, dtype=torch.int32)
+    table[:, :used] = torch.randperm(batch * used, generator=torch.Generator().manual_seed(3)).view(batch, used)
+    lens = torch.tensor([used * 16, 17, 0, 5], dtype=torch.int32)
+
+    def plan(pages: torch.Tensor) -> ops.ClusteredPageDecodePlan:
+        return ops.plan_clustered_page_decode(
+            page_table=pages, seq_lens=lens, num_q_heads=4, num_kv_heads=2, head_dim=64, page_size=16,
+            kv_layout="bf16_kv", use_cache=False)
+
+    tight = plan(table[:, :used])
+    tracemalloc.start()
+    try:
+        wide = plan(table)
+        peak = tracemalloc.get_traced_memory()[1]
+    finally:
+        tracemalloc.stop()
+    assert peak < batch * width  # one byte per page of the table
+    for name, values in tight.device_tensors("cpu").items():
+        assert torch.equal(wide.device_tensors("cpu")[name], values), name
+
+
+@pytest.mark.parametrize("lens", [[0], [0, 0], [-5, 0], [-40, -16]])
+def test_plan_of_requests_without_pages(lens: list[int]) -> None:
+    plan = ops.plan_clustered_page_decode(
+        page_table=torch.zeros((len(lens), 4), dtype=torch.int32), seq_lens=torch.tensor(lens), num_q_heads=4,
+        num_kv_heads=2, head_dim=64, page_size=16, kv_layout="bf16_kv", use_cache=False)
+    assert plan.num_runs == 0
+    assert plan.request_run_offsets_cpu.tolist() == [0] * (len(lens) + 1)
