@@ -391,6 +391,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) w4a16_gemm_tile_kernel(const 
       // one issuer is held by its MMAs the other goes through its waits and commits. (A single issuer
       // spent 1900 of 2700 clocks a step on those.) The stage's activations have landed when its
       // packets are unpacked: the unpack warps wait for the one barrier of both.
+      // Earlier work may still run, for longer than a bounded wait lasts, and the first of those here
+      // ends only after the producer has got past it.
+      pdl_wait_for_prerequisites();
       const uint32_t e = static_cast<uint32_t>(warp) - 1;
       const uint32_t idesc_first =
           tile::idesc(std::is_same<E, BF16>::value, rows < kHalfRows ? rows : kHalfRows);
@@ -452,6 +455,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) w4a16_gemm_tile_kernel(const 
       tile::registers_down<40>();
     }
     // ---- unpack ------------------------------------------------------------------------------
+    pdl_wait_for_prerequisites();  // as the issuers: no bounded wait runs while earlier work does
     const uint32_t e = static_cast<uint32_t>(warp - 4) >> 2;
     const uint32_t quarter = static_cast<uint32_t>(warp) & 3;
     const uint32_t col = (quarter * 32) + lane;
@@ -509,7 +513,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) w4a16_gemm_tile_kernel(const 
     if constexpr (kMoveRegisters) {
       tile::registers_up<184>();
     }
-    // Outputs, slots and tickets are written, and a residual is read, behind earlier work.
+    // Outputs, slots and tickets are written, and a residual is read, behind earlier work; and no
+    // bounded wait runs while it does.
     pdl_wait_for_prerequisites();
     // ---- promote -----------------------------------------------------------------------------
     const uint32_t e = static_cast<uint32_t>(warp - 12) >> 2;

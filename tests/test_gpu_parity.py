@@ -643,6 +643,37 @@ def test_peer_wait_gives_up_and_reports_through_the_status_word() -> None:
         capi.check(lib.fk_w4a16_set_tuning(b"no_such_knob", 1))
 
 
+def test_tile_kernel_waits_for_earlier_work_before_its_bounded_waits() -> None:
+    """A call that waits for another GPU lets the kernels behind it in early and may last longer (2 s
+    here, until it gives up) than their bounded waits (at most 65536 x 20 us): those must not run
+    meanwhile. The batch behind it comes out whole, with the bits of a call of its own."""
+    lib = capi.load_library()
+    shape = LayerShape("t", 128 * 6, 128 * 5, batch=32, dtype="bf16", zero_point=None)
+    problem = make_problem(shape, seed=607)
+    q, alpha, beta, act = (problem[k_].cuda() for k_ in ("q_u8", "alpha", "beta", "activations"))
+    packets = capi_pack(capi, q, alpha, beta, 128)
+    tile_ws = Workspace()  # its own: a call that gave up leaves its workspace to be initialised again
+    assert "gemm_tile" in capi.describe_plan(32, shape.n, shape.k, 128, 1)
+    want = capi_gemv(capi, tile_ws, act, packets, shape.n, shape.k, 128, 1)
+    single = torch.empty((1, shape.n), dtype=torch.bfloat16, device="cuda")
+    signals = torch.zeros(8, dtype=torch.int32, device="cuda")
+    waiting_ws = Workspace().get(capi, 1, shape.n, shape.k, 128)
+    args = capi.GemvArgs()
+    args.activations, args.packets, args.output = act.data_ptr(), packets.data_ptr(), single.data_ptr()
+    args.workspace, args.workspace_bytes = waiting_ws.data_ptr(), waiting_ws.numel()
+    args.batch, args.n, args.k, args.group_size = 1, shape.n, shape.k, 128
+    args.packet_stride_bytes, args.dtype = 8704, 1
+    args.local_signal, args.wait_value = signals.data_ptr(), 2  # one delivery more than will come
+    args.stream = stream_ptr()
+    torch.cuda.synchronize()
+    capi.check(lib.fk_w4a16_set_tuning(b"peer_wait_ms", 2000))
+    capi.check(lib.fk_w4a16_gemv_ex(args))
+    out = capi_gemv(capi, tile_ws, act, packets, shape.n, shape.k, 128, 1)
+    torch.cuda.synchronize()
+    assert capi.device_status() == 2  # the first call's
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
 def _gemv_ex(lib, act, packets, out, shape, code, *, f32=0, residual=None):
     args = capi.GemvArgs()
     ws = WS.get(capi, shape.batch, shape.n, shape.k, shape.group_size)
