@@ -578,6 +578,35 @@ size_t workspace_bytes_for(const Plan& plan, size_t header_bytes = kHeaderBytes)
          ((plan.staged_bytes + 255) & ~size_t{255});
 }
 
+// What the tile kernel needs for any batch up to `batch`: a workspace made for the largest batch
+// serves the smaller ones. A plan's own need falls where the rows are split into one more pass (128
+// rows on 28672 x 8192: 40 MB, 129 rows in two passes of 80: 27 MB), and to nothing where the rule stops
+// wanting the kernel. Up to 64 rows, and from there to 128, it grows with the batch; above, passes of 128
+// rows on every SM bound it.
+size_t tile_workspace_bytes(int batch, int n, int k, int group_size, const DeviceInfo& info) {
+  size_t need = 0;
+  for (const int edge : {64, kTileMaxRows}) {
+    const Plan plan = tile_plan_if_wanted(batch < edge ? batch : edge, n, k, group_size, info);
+    if (plan.stages >= 2 && workspace_bytes_for(plan) > need) {
+      need = workspace_bytes_for(plan);
+    }
+  }
+  if (batch > kTileMaxRows) {
+    Plan plan = tile_plan_if_wanted(batch, n, k, group_size, info);
+    if (plan.stages >= 2) {
+      const long long units = static_cast<long long>(((n / kTileCols) + kTilePair - 1) / kTilePair) * plan.row_tiles;
+      long long ctas = launch_config().ctas > 0 ? launch_config().ctas : info.sm_count;
+      ctas = ctas > 256 ? 256 : ctas;
+      ctas = ctas > units * plan.blocks ? units * plan.blocks : ctas;
+      plan.scratch_bytes = static_cast<size_t>(ctas) * 2 * kTilePair * kTileMaxRows * kTileCols * sizeof(float);
+      plan.staged_bytes =
+          static_cast<size_t>(plan.row_tiles) * plan.blocks * tile_block_bytes(group_size, kTileMaxRows);
+      need = workspace_bytes_for(plan) > need ? workspace_bytes_for(plan) : need;
+    }
+  }
+  return need;
+}
+
 // Opts a kernel in to the device's full dynamic shared memory, once per function and device
 // (minus whatever the kernel declares statically). `flags` must be distinct per instantiation.
 template <class Kernel>
@@ -912,11 +941,8 @@ size_t fk_w4a16_workspace_bytes(int batch, int n, int k, int group_size) {
       make_umma_plan(batch, n, k, group_size, info->sm_count, info->max_smem_optin, launch_config());
   size_t need = workspace_bytes_for(plan);
   need = need > workspace_bytes_for(umma_plan) ? need : workspace_bytes_for(umma_plan);
-  const Plan tile_plan = tile_plan_if_wanted(batch, n, k, group_size, *info);
-  if (tile_plan.stages >= 2) {
-    need = need > workspace_bytes_for(tile_plan) ? need : workspace_bytes_for(tile_plan);
-  }
-  return need;
+  const size_t tile_need = tile_workspace_bytes(batch, n, k, group_size, *info);
+  return need > tile_need ? need : tile_need;
 }
 
 int fk_w4a16_describe_plan(int batch, int n, int k, int group_size, int dtype, char* text,

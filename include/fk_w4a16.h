@@ -67,7 +67,9 @@ FK_W4A16_API int fk_w4a16_group_sums(const void* activations, float* sums, int b
 
 /* Scratch the fused GEMV needs for a problem, in bytes (a multiple of 256; never 0). The caller
  * allocates it on the device, zero-fills it ONCE (fk_w4a16_workspace_init or cudaMemset) and may
- * then reuse it for any number of calls whose requirement is not larger. Calls that run
+ * then reuse it for any number of calls whose requirement is not larger. For one layer it never
+ * falls as the batch grows: a workspace made for the largest batch serves every smaller one on the
+ * kernel that a workspace of its own would get. Calls that run
  * concurrently on the GPU need separate workspaces. */
 FK_W4A16_API size_t fk_w4a16_workspace_bytes(int batch, int n, int k, int group_size);
 FK_W4A16_API int fk_w4a16_workspace_init(void* workspace, size_t workspace_bytes, void* stream);

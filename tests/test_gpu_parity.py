@@ -891,6 +891,45 @@ def test_gemm_tile_batches(group: int, dtype: str, batch: int, tiles: int, featu
         capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
 
 
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize(("n", "k"), [(28672, 8192), (4096, 4096), (2048, 4096), (1024, 1024), (512, 8192), (128, 128),
+                                      (1024, 28672), (128256, 4096)])
+def test_workspace_for_a_batch_serves_the_smaller_ones(n: int, k: int, group: int) -> None:
+    lib = capi.load_library()
+    needs = [int(lib.fk_w4a16_workspace_bytes(batch, n, k, group)) for batch in range(1, 521)]
+    falls = [batch + 1 for batch in range(1, 520) if needs[batch] < needs[batch - 1]]
+    assert not falls
+
+
+def test_workspace_for_a_larger_batch_runs_the_same_kernel() -> None:
+    """128 rows on a workspace made for 144 (two passes of 80 rows): the bits of the tile kernel, as on a
+    workspace made for 128, and not those of the kernel that takes calls whose workspace is too small."""
+    lib = capi.load_library()
+    n = k = 4096
+    problem = make_problem(LayerShape("t", n, k, batch=128, dtype="bf16", zero_point=None), seed=144)
+    q, alpha, beta, act = (problem[key].cuda() for key in ("q_u8", "alpha", "beta", "activations"))
+    packets = capi_pack(capi, q, alpha, beta, 128)
+
+    def run(rows_of_workspace: int) -> torch.Tensor:
+        ws = Workspace()
+        ws.get(capi, rows_of_workspace, n, k, 128)
+        out = torch.full((128, n), float("nan"), dtype=act.dtype, device="cuda")
+        capi.check(lib.fk_w4a16_gemv(act.data_ptr(), packets.data_ptr(), out.data_ptr(), ws.buffer.data_ptr(),
+                                     ws.buffer.numel(), 128, n, k, 128, 8704, 1, stream_ptr()))
+        torch.cuda.synchronize()
+        return out.view(torch.int16)
+
+    want = run(128)
+    capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", 0))
+    try:
+        former = run(128)
+    finally:
+        capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
+    assert not torch.equal(former, want)  # the two kernels round differently somewhere in 524288 outputs
+    assert torch.equal(run(144), want)
+    assert torch.equal(run(512), want)
+
+
 @pytest.mark.parametrize(("n", "k", "batch"), [(4096, 4096, 8), (28672, 8192, 16), (4096, 14336, 8)])
 def test_gemm_tensor_core_layer_shapes(n: int, k: int, batch: int) -> None:
     shape = LayerShape("t", n, k, batch=batch, dtype="bf16", zero_point=None)
