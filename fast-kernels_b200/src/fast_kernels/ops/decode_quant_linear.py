@@ -41,6 +41,7 @@ LAYOUT_TO_GROUP_SIZE: dict[str, int] = {
 # buffers a kernel writes): tensors are reused across calls and never freed while the process
 # lives, so a kernel still in flight can never see its scratch recycled.
 _WORKSPACES: dict[tuple[int, int], Any] = {}
+_OUTGROWN_WORKSPACES: list[Any] = []  # each less than half its successor's size
 _WEIGHT_BUFFERS: dict[tuple[int, int, int, Any], Any] = {}
 _VENDOR_WORKSPACES: dict[tuple[int, int], Any] = {}
 _PARTIALS: dict[tuple[int, int, int, int, int], Any] = {}
@@ -154,14 +155,16 @@ def _resolve_arc_impl(device: Any, impl: str | None) -> str:
 
 
 def _gemv_workspace(native: Any, device: Any, stream_ptr: int, need: int) -> Any:
-    """Zero-initialised GEMV scratch for (device, stream); grows, never shrinks."""
+    """Zero-initialised GEMV scratch for (device, stream); grows, never shrinks. An outgrown buffer is
+    kept: a CUDA graph recorded with it goes on writing to it."""
     torch = _require_torch()
     key = (_device_index(device), stream_ptr)
     buffer = _WORKSPACES.get(key)
     if buffer is None or buffer.numel() < need:
-        # Sized generously so that shape changes do not reallocate; the old tensor is dropped only
-        # after the allocator has ordered its reuse behind work already queued on this stream.
-        buffer = torch.zeros(max(need * 2, 4 << 20), device=device, dtype=torch.uint8)
+        if buffer is not None:
+            _OUTGROWN_WORKSPACES.append(buffer)
+        # Sized generously so that shape changes do not reallocate: the first holds every layer up to 16 rows.
+        buffer = torch.zeros(max(need * 2, 8 << 20), device=device, dtype=torch.uint8)
         _WORKSPACES[key] = buffer
     return buffer
 

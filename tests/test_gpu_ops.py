@@ -6,6 +6,8 @@ are added as extra parameters."""
 
 from __future__ import annotations
 
+import importlib
+
 import numpy as np
 import pytest
 import torch
@@ -222,3 +224,40 @@ def test_native_forward_can_be_captured_after_one_warm_up_call() -> None:
             with torch.cuda.graph(graph2, stream=fresh):
                 call(fresh)
     torch.cuda.synchronize()
+
+
+def test_a_recorded_call_outlives_the_growth_of_its_workspace() -> None:
+    """Calls of up to 16 rows share the workspace that the first one made. A larger batch makes a larger
+    one, and the graph that was recorded with the former still owns what it writes to."""
+    ops = importlib.import_module("fast_kernels.ops.decode_quant_linear")
+    n = k = 4096
+    cpu = _inputs(31, 1, n, k, 128, 0.005, 0.015)
+    activations, q_u8, alpha, beta = (t.cuda() for t in cpu)
+    packets = pack_arc_w4a16_packets(q_u8, alpha, beta, group_size=128)
+    out = torch.zeros((1, n), dtype=torch.float16, device="cuda")
+
+    def forward(rows: torch.Tensor, output: torch.Tensor | None = None) -> torch.Tensor:
+        return arc_w4a16_forward(rows, packets, n=n, k=k, group_size=128, output=output)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        forward(activations, out)
+        key = (torch.cuda.current_device(), side.cuda_stream)
+        first = ops._WORKSPACES[key]
+        forward(activations.expand(16, k).contiguous())
+        assert ops._WORKSPACES[key] is first
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            forward(activations, out)
+        address, size = first.data_ptr(), first.numel()
+        del first
+        forward(activations.expand(256, k).contiguous())
+        assert ops._WORKSPACES[key].data_ptr() != address
+        fresh = [torch.full((size,), 255, dtype=torch.uint8, device="cuda") for _ in range(4)]
+        assert all(abs(buffer.data_ptr() - address) >= size for buffer in fresh)  # its memory is not given out
+        out.zero_()
+        graph.replay()
+    side.synchronize()
+    assert all(bool((buffer == 255).all()) for buffer in fresh)
+    _assert_matches(out, cpu, 128)
