@@ -31,13 +31,13 @@ void* as_ptr(std::uintptr_t value) { return reinterpret_cast<void*>(value); }
 // per (device, stream): calls on one stream are ordered and can share it, calls on different
 // streams may overlap and must not. The rule for callers:
 //   * the FIRST call on a (device, stream) pair allocates the pair's workspace (cudaMalloc, one
-//     buffer of kFixedWorkspaceBytes, enough for every layer shape at batches up to 16) -- make
+//     buffer of kFixedWorkspaceBytes, enough for batches up to 64 on layers of up to 65536 features) -- make
 //     that call outside stream capture; every later call allocates nothing and can be captured;
-//   * a problem that needs more than that (batches far above 16) makes the buffer grow: the
+//   * a problem that needs more than that (batches far above 64) makes the buffer grow: the
 //     stream is synchronised, the old buffer freed, a larger one allocated. Never under capture:
 //     there the call fails with std::runtime_error instead.
 // Buffers live until the process ends.
-constexpr std::size_t kFixedWorkspaceBytes = std::size_t{16} << 20;
+constexpr std::size_t kFixedWorkspaceBytes = std::size_t{32} << 20;
 
 struct OwnedWorkspace {
   void* ptr = nullptr;

@@ -226,6 +226,35 @@ def test_native_forward_can_be_captured_after_one_warm_up_call() -> None:
     torch.cuda.synchronize()
 
 
+def test_native_forward_of_a_batch_can_be_captured_after_a_single_row() -> None:
+    """The workspace that the first call on a stream allocates holds batches of 80 rows on a 4096 x 4096
+    layer: such a call may be the first of its size inside a capture."""
+    native = native_module()
+    n = k = 4096
+    cpu = _inputs(78, 80, n, k, 128, 0.005, 0.015)
+    activations, q_u8, alpha, beta = (t.cuda() for t in cpu)
+    packets = pack_arc_w4a16_packets(q_u8, alpha, beta, group_size=128)
+    out = torch.zeros((80, n), dtype=torch.float16, device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+
+    def call(batch: int) -> None:
+        native.arc_w4a16_forward(activations_ptr=activations.data_ptr(), packets_ptr=packets.data_ptr(),
+                                 group_sums_ptr=0, output_ptr=out.data_ptr(), batch=batch, n=n, k=k,
+                                 group_size=128, packet_stride_bytes=8704, stream_ptr=side.cuda_stream)
+
+    with torch.cuda.stream(side):
+        call(1)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            call(80)
+        out.zero_()
+        graph.replay()
+    side.synchronize()
+    _assert_matches(out, cpu, 128)
+
+
 def test_a_recorded_call_outlives_the_growth_of_its_workspace() -> None:
     """Calls of up to 16 rows share the workspace that the first one made. A larger batch makes a larger
     one, and the graph that was recorded with the former still owns what it writes to."""
