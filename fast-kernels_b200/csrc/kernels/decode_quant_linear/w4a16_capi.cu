@@ -968,11 +968,16 @@ int fk_w4a16_describe_plan(int batch, int n, int k, int group_size, int dtype, c
                        : plan.wmma          ? "w4a16_gemv_wmma_kernel"
                        : plan.cluster_size > 1 ? "w4a16_gemv_cluster_kernel"
                                                : "w4a16_gemv_stream_kernel";
+  // The tile kernel's row tiles are units of its CTAs' runs, not of the grid, and its instances are by
+  // the rows that they have room for.
   std::ostringstream oss;
-  oss << kernel << "<" << group_size << ", " << plan.m_tile << ", "
-      << (dtype == FK_W4A16_DTYPE_BF16 ? "UnpackBF16" : "UnpackF16") << "> grid=" << plan.grid_x << "x"
-      << plan.row_tiles << " cluster=" << plan.cluster_size << " warps=" << plan.warps
+  oss << kernel << "<" << group_size << ", " << (plan.tile ? tile_rows_template(plan.m_tile) : plan.m_tile) << ", "
+      << (plan.tile ? "" : "Unpack") << (dtype == FK_W4A16_DTYPE_BF16 ? "BF16" : "F16") << "> grid=" << plan.grid_x
+      << "x" << (plan.tile ? 1 : plan.row_tiles) << " cluster=" << plan.cluster_size << " warps=" << plan.warps
       << " stages=" << plan.stages << " smem=" << plan.smem_bytes;
+  if (plan.tile) {
+    oss << " rows=" << plan.m_tile << " row_tiles=" << plan.row_tiles;
+  }
   const std::string line = oss.str();
   if (line.size() + 1 > capacity) {
     return fail(FK_W4A16_ERR_INVALID_ARGUMENT, "text buffer is too small");

@@ -891,6 +891,19 @@ def test_gemm_tile_batches(group: int, dtype: str, batch: int, tiles: int, featu
         capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
 
 
+@pytest.mark.parametrize(("batch", "instance", "rows", "row_tiles"), [
+    (16, 16, 16, 1), (40, 64, 48, 1), (128, 128, 128, 1), (129, 128, 80, 2), (256, 128, 128, 2)])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+def test_describe_plan_names_the_launch_of_the_tile_kernel(batch: int, instance: int, rows: int, row_tiles: int,
+                                                           dtype: str) -> None:
+    """The instance that runs and a grid of one row of CTAs, at most one per SM, however many row tiles."""
+    text = capi.describe_plan(batch, 28672, 8192, 128, oracle.dtype_code(dtype))
+    element = {"fp16": "F16", "bf16": "BF16"}[dtype]
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count
+    assert text.startswith(f"w4a16_gemm_tile_kernel<128, {instance}, {element}> grid={ctas}x1 cluster=1 warps=20 ")
+    assert text.endswith(f" rows={rows} row_tiles={row_tiles}")
+
+
 @pytest.mark.parametrize("group", [32, 64, 128])
 @pytest.mark.parametrize(("n", "k"), [(28672, 8192), (4096, 4096), (2048, 4096), (1024, 1024), (512, 8192), (128, 128),
                                       (1024, 28672), (128256, 4096)])
