@@ -511,6 +511,10 @@ bool tile_wanted(int batch, int n, int k) {
   if (min_batch >= 0) {
     return min_batch > 0 && batch >= min_batch;
   }
+  // A caller who sets the other kernels' threshold or warps per CTA means those kernels.
+  if (tuning().mma_min_batch > 0 || launch_config().warps > 0) {
+    return false;
+  }
   return batch > 8 && (batch <= 64 || static_cast<long long>(n) * k >= 6ll << 20);
 }
 

@@ -891,6 +891,29 @@ def test_gemm_tile_batches(group: int, dtype: str, batch: int, tiles: int, featu
         capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
 
 
+def test_settings_of_the_other_kernels_keep_batches_on_them() -> None:
+    """"mma_min_batch" and a warp count are choices for kernels other than the tile kernel: they act on
+    every batch, unless "tile_min_batch" asks for the tile kernel."""
+    lib = capi.load_library()
+    layer = (4096, 4096, 128, 1)
+    assert "gemm_tile" in capi.describe_plan(16, *layer)
+    try:
+        capi.check(lib.fk_w4a16_set_tuning(b"mma_min_batch", 16))
+        assert "gemm_mma" in capi.describe_plan(16, *layer)
+        assert "gemv_" in capi.describe_plan(15, *layer)
+        capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", 12))
+        assert "gemm_tile" in capi.describe_plan(15, *layer)
+        capi.check(lib.fk_w4a16_set_tuning(b"mma_min_batch", 0))
+        capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
+        capi.check(lib.fk_w4a16_set_launch_config(4, 0, 0))
+        text = capi.describe_plan(16, *layer)
+        assert "gemm_mma" in text and " warps=4 " in text
+    finally:
+        capi.check(lib.fk_w4a16_set_tuning(b"mma_min_batch", 0))
+        capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
+        capi.check(lib.fk_w4a16_set_launch_config(0, 0, 0))
+
+
 @pytest.mark.parametrize(("batch", "instance", "rows", "row_tiles"), [
     (16, 16, 16, 1), (40, 64, 48, 1), (128, 128, 128, 1), (129, 128, 80, 2), (256, 128, 128, 2)])
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
