@@ -859,7 +859,7 @@ def test_gemv_ex_silu_mul_refusals() -> None:
 @pytest.mark.parametrize("group", [32, 64, 128])
 @pytest.mark.parametrize("batch", [5, 8, 9, 16, 19])
 def test_gemm_tensor_core_batches(group: int, batch: int, dtype: str) -> None:
-    """Batches above 4 take the MMA kernel (rows in tiles of 8 or 16, the last one padded)."""
+    """Batches above 4 on the tensor cores: 5 and 8 on mma.sync, above 8 the tile kernel."""
     shape = LayerShape("t", 128 * 5, group * 9, group_size=group, batch=batch, dtype=dtype,
                        zero_point=None, scale_range=(0.001, 0.05))
     _check_gemv(make_problem(shape, seed=13 * group + batch), shape, oracle.dtype_code(dtype))
@@ -889,6 +889,179 @@ def test_gemm_tile_batches(group: int, dtype: str, batch: int, tiles: int, featu
         _check_gemv(make_problem(shape, seed=17 * group + batch), shape, oracle.dtype_code(dtype))
     finally:
         capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
+
+
+@pytest.fixture
+def _no_tile_kernel():
+    capi.check(capi.load_library().fk_w4a16_set_tuning(b"tile_min_batch", 0))
+    yield
+    capi.check(capi.load_library().fk_w4a16_set_tuning(b"tile_min_batch", -1))
+
+
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize("batch", [9, 16, 19, 65])
+def test_gemm_mma_batches_above_8(_no_tile_kernel, group: int, batch: int, dtype: str) -> None:
+    """The mma.sync kernel in passes of 16 rows, the last one padded: gated and multi-GPU calls, small
+    layers above 64 rows and calls with little workspace still take it."""
+    shape = LayerShape("t", 128 * 5, group * 9, group_size=group, batch=batch, dtype=dtype,
+                       zero_point=None, scale_range=(0.001, 0.05))
+    assert "gemm_mma" in capi.describe_plan(batch, shape.n, shape.k, group, oracle.dtype_code(dtype))
+    _check_gemv(make_problem(shape, seed=13 * group + batch), shape, oracle.dtype_code(dtype))
+
+
+def test_gemm_mma_of_a_large_layer_at_16_rows(_no_tile_kernel) -> None:
+    shape = LayerShape("t", 28672, 8192, batch=16, dtype="bf16", zero_point=None)
+    assert "gemm_mma" in capi.describe_plan(16, shape.n, shape.k, 128, 1)
+    test_gemm_tensor_core_layer_shapes(shape.n, shape.k, shape.batch)
+
+
+@pytest.mark.parametrize(("batch", "kernel"), [(64, "gemm_tile"), (65, "gemm_mma"), (128, "gemm_mma"), (256, "gemm_mma")])
+def test_small_layer_by_the_rule(batch: int, kernel: str) -> None:
+    shape = LayerShape("t", 512, 1024, batch=batch, dtype="bf16", zero_point=None)
+    assert kernel in capi.describe_plan(batch, shape.n, shape.k, 128, 1)
+    _check_gemv(make_problem(shape, seed=batch), shape, 1)
+
+
+@pytest.mark.parametrize(("batch", "dtype"), [(16, "bf16"), (33, "fp16")])
+def test_gemv_ex_fused_silu_mul_above_8_rows(batch: int, dtype: str) -> None:
+    """The gated epilogue stays on the mma.sync kernel, whatever the batch."""
+    lib = capi.load_library()
+    n, k = 128 * 6, 128 * 5
+    code = oracle.dtype_code(dtype)
+    problem = make_problem(LayerShape("t", n, k, batch=batch, dtype=dtype, zero_point=None), seed=77 + batch)
+    q, alpha, beta, act = (problem[key].cuda() for key in ("q_u8", "alpha", "beta", "activations"))
+    packets = capi_pack(capi, q, alpha, beta, 128)
+    ws = WS.get(capi, batch, n, k, 128)
+    outs = [torch.full((batch, n // 2), float("nan"), dtype=act.dtype, device="cuda") for _ in range(2)]
+    for out in outs:
+        args = capi.GemvArgs()
+        args.activations, args.packets, args.output = act.data_ptr(), packets.data_ptr(), out.data_ptr()
+        args.workspace, args.workspace_bytes = ws.data_ptr(), ws.numel()
+        args.batch, args.n, args.k, args.group_size = batch, n, k, 128
+        args.packet_stride_bytes, args.dtype = 8704, code
+        args.epilogue = capi.EPILOGUE_SILU_MUL
+        args.stream = stream_ptr()
+        capi.check(lib.fk_w4a16_gemv_ex(args))
+    torch.cuda.synchronize()
+    y64 = oracle.gemv_f64(oracle.bits_of(problem["activations"]), problem["q_u8"].numpy(),
+                          oracle.bits_of(problem["alpha"]), oracle.bits_of(problem["beta"]), 128, code)
+    gate, up = y64[:, : n // 2], y64[:, n // 2:]
+    assert oracle.max_rel_err(outs[0].double().cpu().numpy(), gate / (1.0 + np.exp(-gate)) * up) <= GEMV_REL_TOL
+    assert torch.equal(outs[0].view(torch.int16), outs[1].view(torch.int16))
+
+
+def _tile_call(batch: int, seed: int, n: int = 128 * 5, k: int = 128 * 9):
+    """A bf16 problem on the device and a function that calls fk_w4a16_gemv_ex on it."""
+    lib = capi.load_library()
+    problem = make_problem(LayerShape("t", n, k, batch=batch, dtype="bf16", zero_point=None), seed=seed)
+    q, alpha, beta, act = (problem[key].cuda() for key in ("q_u8", "alpha", "beta", "activations"))
+    packets = capi_pack(capi, q, alpha, beta, 128)
+    ws = Workspace().get(capi, batch, n, k, 128)
+    assert "gemm_tile" in capi.describe_plan(batch, n, k, 128, 1)
+
+    def call(out: torch.Tensor, rows: torch.Tensor = act, workspace_bytes: int = ws.numel(), **options: int) -> None:
+        args = capi.GemvArgs()
+        args.activations, args.packets, args.output = rows.data_ptr(), packets.data_ptr(), out.data_ptr()
+        args.workspace, args.workspace_bytes = ws.data_ptr(), workspace_bytes
+        args.batch, args.n, args.k, args.group_size = batch, n, k, 128
+        args.packet_stride_bytes, args.dtype = 8704, 1
+        for name, value in options.items():
+            setattr(args, name, value)
+        args.stream = stream_ptr()
+        capi.check(lib.fk_w4a16_gemv_ex(args))
+
+    plain = torch.full((batch, n), float("nan"), dtype=torch.bfloat16, device="cuda")
+    call(plain)
+    torch.cuda.synchronize()
+    assert bool(plain.isfinite().all())
+    return act, call, plain
+
+
+@pytest.mark.parametrize("batch", [17, 70])
+@pytest.mark.parametrize("fp32", [0, 1])
+def test_tile_kernel_places_its_output(batch: int, fp32: int) -> None:
+    """output_ld / output_col0, with and without a residual in the same place: the bits of the plain
+    call in their columns, and nothing beside them."""
+    _, call, plain = _tile_call(batch, seed=5, n=128 * 49, k=128 * 9)
+    n = plain.shape[1]
+    ld, col0 = n + 260, 132
+    dtype = torch.float32 if fp32 else torch.bfloat16
+    wide = torch.full((batch, ld), -7.0, dtype=dtype, device="cuda")
+    call(wide, output_ld=ld, output_col0=col0, output_f32=fp32)
+    residual = torch.randn((batch, ld), generator=torch.Generator().manual_seed(5)).to(torch.bfloat16).cuda()
+    added = torch.full((batch, ld), -7.0, dtype=dtype, device="cuda")
+    call(added, output_ld=ld, output_col0=col0, output_f32=fp32, residual=residual.data_ptr())
+    y32 = torch.empty((batch, n), dtype=torch.float32, device="cuda")
+    call(y32, output_f32=1)
+    torch.cuda.synchronize()
+    inside = slice(col0, col0 + n)
+    assert torch.equal(wide[:, inside], y32 if fp32 else plain)
+    assert torch.equal(added[:, inside], (y32 + residual[:, inside].float()).to(dtype))
+    for out in (wide, added):
+        assert bool((out[:, :col0] == -7.0).all()) and bool((out[:, col0 + n:] == -7.0).all())
+
+
+def test_small_workspace_takes_the_former_kernel() -> None:
+    """A workspace that holds the mma.sync plan only is accepted, and that kernel runs."""
+    lib = capi.load_library()
+    batch, n, k = 64, 4096, 4096
+    act, call, plain = _tile_call(batch, seed=6, n=n, k=k)
+    capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", 0))
+    try:
+        small = int(lib.fk_w4a16_workspace_bytes(batch, n, k, 128))
+        former = torch.full_like(plain, float("nan"))
+        call(former)
+    finally:
+        capi.check(lib.fk_w4a16_set_tuning(b"tile_min_batch", -1))
+    assert small < int(lib.fk_w4a16_workspace_bytes(batch, n, k, 128))
+    out = torch.full_like(plain, float("nan"))
+    call(out, workspace_bytes=small)
+    again = torch.full_like(plain, float("nan"))
+    call(again)  # the whole workspace: the tile kernel, behind the other one's use of the same bytes
+    torch.cuda.synchronize()
+    assert torch.equal(out, former) and not torch.equal(out, plain)
+    assert torch.equal(again, plain)
+    with pytest.raises(ValueError, match="smaller than the required"):
+        call(out, workspace_bytes=1 << 20)
+
+
+def test_tile_calls_replay_in_a_graph() -> None:
+    """Two dependent-launch pairs recorded and replayed on new activations."""
+    act, call, plain = _tile_call(70, seed=7, n=128 * 49)
+    first, second = torch.empty_like(plain), torch.empty_like(plain)
+    graph = torch.cuda.CUDAGraph()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        with torch.cuda.graph(graph, stream=side):
+            call(first)
+            call(second)
+    torch.cuda.current_stream().wait_stream(side)
+    saved = act.clone()
+    for scale in (1.0, 2.0):  # a power of two: every product and sum scales exactly
+        act.copy_(saved * scale)
+        first.fill_(float("nan"))
+        second.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(first, plain * scale) and torch.equal(second, plain * scale)
+
+
+@pytest.mark.parametrize("batch", [40, 129])
+def test_tile_kernel_keeps_infinities_and_nans_in_their_rows(batch: int) -> None:
+    act, call, plain = _tile_call(batch, seed=8, n=128 * 49, k=128 * 9)
+    dirty = act.clone()
+    dirty[3, 5] = float("inf")
+    dirty[17, 1151] = float("nan")
+    dirty[batch - 1, 600] = float("-inf")
+    out = torch.zeros_like(plain)
+    call(out, dirty)
+    torch.cuda.synchronize()
+    clean = torch.ones(batch, dtype=torch.bool)
+    clean[[3, 17, batch - 1]] = False
+    assert torch.equal(out[clean.cuda()], plain[clean.cuda()])
+    assert not bool(out[~clean.cuda()].isfinite().any())
 
 
 def test_settings_of_the_other_kernels_keep_batches_on_them() -> None:
