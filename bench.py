@@ -12,11 +12,13 @@ seeded shapes and value distributions, no checkpoint.
 
 The step is captured once as a CUDA graph of 128 launches of the library's C-ABI entry point
 (`fk_w4a16_gemv`) and replayed; timing is by CUDA events on the launching stream between a barrier
-and a device synchronisation, maximum over ranks. One JSON line is printed by rank 0.
+and a device synchronisation, maximum over ranks. One JSON line with the headline is printed by rank 0; the
+whole record, with the tables and extra keys described below, goes to stderr as one line of JSON
+behind "details: ".
 
 The timed region of K steps is repeated (`--regions`, default 15); `value` is the median region,
 the spread is reported beside it. `roofline` names the kernel with the largest share of the step
-and carries one entry per kernel (`kernels`) and per layer shape (`per_layer`).
+and, in the whole record, carries one entry per kernel (`kernels`) and per layer shape (`per_layer`).
 
 `e2e` measures the same work through the C-ABI entry point that takes HOST buffers
 (`fk_w4a16_gemv_host`), one call per GEMV: every call pulls its activations from pinned host
@@ -921,6 +923,36 @@ def _kernel_table(capi, per_layer: list[dict], ms_per_step: float) -> list[dict]
     return sorted(out, key=lambda e: -e["share_of_step"])
 
 
+def _rounded(value):
+    """Floats to six significant digits, at any depth."""
+    if isinstance(value, float):
+        return float(f"{value:.6g}")
+    if isinstance(value, dict):
+        return {key: _rounded(item) for key, item in value.items()}
+    return [_rounded(item) for item in value] if isinstance(value, list) else value
+
+
+def _headline(line: dict) -> dict:
+    """What is printed on stdout: the headline, its clocks, roofline, end-to-end and CPU figures, and
+    errors, in less than 2500 characters (readers keep the end of the output only). Tables per layer,
+    kernel and configuration are left to the whole record on stderr."""
+    short = {key: value for key, value in line.items()
+             if key not in ("pack", "layer_chain", "sharded_layers", "configs", "reference_gpu", "page_decode", "regions")}
+    short["regions"] = {key: line["regions"][key] for key in ("count", "value_min", "value_max")}
+    short["roofline"] = {key: line["roofline"][key] for key in ("bound", "kernel", "achieved", "peak", "unit", "frac",
+                                                                "algorithmic_bytes_per_launch", "traffic")}
+    short["roofline"]["step_frac"] = line["roofline"]["step"]["frac"]
+    short["e2e"] = {key: value for key, value in line["e2e"].items() if key != "eager"}
+    for key, value in line.items():
+        if isinstance(value, dict) and "error" in value:
+            short[key] = {"error": value["error"][:120]}
+    failed = sum("failed" in row for row in line.get("sharded_layers", {}).get("results", []))
+    failed += sum("failed" in row for row in line.get("page_decode", {}).get("results", []))
+    if failed:
+        short["failed_checks"] = failed
+    return _rounded(short)
+
+
 def run_ours(args) -> int:
     import torch
     import torch.distributed as dist
@@ -1107,7 +1139,9 @@ def run_ours(args) -> int:
         line.update(extra)
         if world == 1 and not args.no_cpu_baseline:
             line["cpu_baseline"] = _cpu_baseline_leg()
-        print(json.dumps(line), flush=True)
+        # the whole record beside it, so that the one line on stdout stays short
+        print("details: " + json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(_headline(line)), flush=True)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()

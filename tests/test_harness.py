@@ -109,3 +109,37 @@ def test_result_bundle_round_trip(tmp_path: Path) -> None:
     loaded = load_result_bundle(tmp_path)
     assert loaded.schema_version == 2 and loaded.cases[0].metrics["hbm_gbs"] == 2100.0
     assert "decode/w4a16_linear" in (tmp_path / "summary.md").read_text()
+
+
+def test_headline_line_of_the_benchmark_stays_short() -> None:
+    """The line on stdout keeps the headline keys and stays below 2500 characters, however long the tables
+    of the whole record are."""
+    import bench
+
+    x = 1234.5678901234567
+    tables = {"results": [{"shape": "gqa4_batch32_4k_page16", "us_per_call": x, "failed": "x"}] * 40}
+    kernel = "w4a16_gemv_cluster_kernel<128, 1, UnpackBF16>"
+    line = {
+        "metric": bench.METRIC, "value": x, "unit": bench.UNIT, "n_gpus": 8, "steps": 100, "warmup": 5,
+        "ms_per_step": x, "us_per_call": x, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+        "dtype": "bf16", "data": "synthetic", "config": bench._config(8),
+        "regions": {"count": 15, "steps_each": 100, "ms_per_step_median": x, "ms_per_step_min": x,
+                    "ms_per_step_max": x, "value_min": x, "value_max": x},
+        "roofline": {"bound": "hbm", "kernel": kernel, "achieved": x, "peak": x, "unit": "GB/s", "frac": x,
+                     "peak_source": "text " * 20, "algorithmic_bytes_per_launch": x, "traffic": x,
+                     "step": {"frac": x, "note": "text"}, "kernels": [{"name": kernel}] * 4, "per_layer": [{}] * 4},
+        "e2e": {"value": x, "unit": bench.UNIT, "h2d_bytes_per_step": 10**6, "d2h_bytes_per_step": 10**7,
+                "us_per_call": x, "steps": 20, "api": "text " * 40, "eager": {"value": x, "note": "text"}},
+        "gpu_launches": 12800, "pack": tables, "layer_chain": {"value": x}, "sharded_layers": tables,
+        "clocks": {"sm_mhz": x, "sm_max_mhz": x, "reasons": ["sw_power_cap"], "samples": 1000},
+        "configs": tables, "reference_gpu": tables, "page_decode": {"error": "text " * 60},
+        "cpu_baseline": {"value": x, "unit": bench.UNIT, "cores": 16, "kind": "port", "sample": "text " * 30,
+                         "us_per_call": x},
+    }
+    short = bench._headline(line)
+    assert len(json.dumps(short)) < 2500
+    assert {"metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks", "roofline",
+            "cpu_baseline"} <= short.keys()
+    assert short["value"] == 1234.57 and short["e2e"]["h2d_bytes_per_step"] == 10**6
+    assert short["failed_checks"] == 40 and short["page_decode"]["error"]
