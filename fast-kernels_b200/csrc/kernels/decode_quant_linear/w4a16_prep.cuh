@@ -9,10 +9,12 @@ namespace fk_w4a16 {
 // ---------------------------------------------------------------------------------------------
 // pack: row-major nibbles q[n, k/2] + alpha/beta[n, k/G]  ->  ARC packets.
 // Same bytes as the reference's pack_arc_packets_kernel (arc_w4a16.cu:87-122). One CTA of 128
-// threads builds a run of neighbouring packets; thread c reads column c's G/2 bytes with 128-bit
-// loads and writes word r to packet_words[r * 128 + c], so every store instruction of a warp is one
-// contiguous 128-byte line. Neighbouring groups share the 32-byte sectors of a row's scales: in a
-// run they are read from L2 once instead of once per 2 bytes.
+// threads builds one packet at a time; thread c reads column c's G/2 bytes with 128-bit loads and
+// writes word r to packet_words[r * 128 + c], so every store instruction of a warp is one
+// contiguous 128-byte line. Neighbouring packets, whose groups lie in the same sectors of a row, are
+// built at the same time by neighbouring CTAs. 28672 x 4096, inputs from HBM, groups of 128 / 64 / 32:
+// 26.6 / 37.6 / 55.7 us (19.1 / 20.2 / 22.4 for the bytes at the measured HBM rate), and 33.3 / 39.4 /
+// 58.7 us with a run of neighbouring packets for each CTA.
 // ---------------------------------------------------------------------------------------------
 template <int G>
 __global__ void __launch_bounds__(128) pack_packets_kernel(const uint8_t* __restrict__ q,
@@ -23,8 +25,7 @@ __global__ void __launch_bounds__(128) pack_packets_kernel(const uint8_t* __rest
   constexpr int kWordRows = G / 8;
   constexpr int kVecs = kWordRows / 4;  // 128-bit loads per column
   const int c = static_cast<int>(threadIdx.x);
-  const long long run_end = (total_packets * (blockIdx.x + 1ll)) / gridDim.x;
-  for (long long pkt = (total_packets * blockIdx.x) / gridDim.x; pkt < run_end; ++pkt) {
+  for (long long pkt = blockIdx.x; pkt < total_packets; pkt += gridDim.x) {
     const long long tile = pkt / num_groups;
     const int group = static_cast<int>(pkt % num_groups);
     const long long row = (tile * kTileCols) + c;
@@ -92,8 +93,8 @@ __global__ void __launch_bounds__(256) dequant_rowmajor_kernel(const uint8_t* __
 // One CTA expands a packet at a time through shared memory: bound by its stores (4 bytes out per
 // byte in), which therefore go out as whole rows of the group, G * 2 contiguous bytes, 16 per
 // thread. (Stored straight from the packet's column order, every 16 bytes went to another row: half
-// a sector each; packing and expanding a 28672 x 4096 layer took 188 us together, now 88, of which
-// HBM needs 63.) The pitch lets the G / 8 words of the rows of a warp be read without conflicts.
+// a sector each; 28672 x 4096, groups of 128: 155 us, now 55.7, of which the bytes need 45 at the
+// measured HBM rate; groups of 64 / 32: 154 / 149, now 61.5 / 64.3.) The pitch lets the G / 8 words of the rows of a warp be read without conflicts.
 // The packets are only known to be 4-byte aligned, hence 32-bit loads.
 template <int G, class E>
 __global__ void __launch_bounds__(256) dequant_packets_kernel(const uint8_t* __restrict__ packets,
