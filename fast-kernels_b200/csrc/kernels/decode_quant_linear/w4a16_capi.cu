@@ -498,11 +498,17 @@ Plan make_umma_plan(int batch, int n, int k, int group_size, int sm_count, int m
 
 // Which problems take the tile kernel by default (FK_W4A16_TILE_MIN_BATCH overrides the rule with a
 // smallest batch; 0 there means "never"). Above 8 rows the mma.sync kernel reads the layer once per
-// 16 rows (28672 x 8192, bf16: 58 / 112 / 221 / 862 us at 16 / 32 / 64 / 256 rows, against 51 / 57 /
-// 68 / 204 here). Its passes run side by side where the layer is too small to fill the chip with
+// 16 rows (28672 x 8192, bf16, groups of 128: 58 / 112 / 221 / 862 us at 16 / 32 / 64 / 256 rows, against
+// 51 / 57 / 68 / 204 here). Its passes run side by side where the layer is too small to fill the chip with
 // one, which is worth more above 64 rows (512 x 1024, 128 rows: 18 us against 28; 1024 x 4096: 34
 // against 39), and no longer at 2048 x 4096 (45 against 39). At 8 rows and fewer the mma.sync
 // kernel keeps its lead (28672 x 8192: 34 us against 50).
+// Compared on sixteen layers from 128 x 128 to 28672 x 4096, groups of 32, 64 and 128, bf16 and fp16, 9
+// to 256 rows. Where the rule takes this kernel it is 1.0 to 5 times as fast, but for four cells of
+// 0.94 to 0.98 (groups of 128: 512 x 512 at 64 rows, 2048 x 4096 at 65; of 64: 4096 x 512 at 64; of 32:
+// 4096 x 512 at 33). The line above 64 rows is the one for groups of 128 up to 128 rows: smaller groups
+// and more rows would gain on smaller layers too (4096 x 1024, 256 rows, groups of 32 / 64 / 128:
+// 146 / 72 / 48 us on the mma.sync kernel, 35 / 32 / 30 here).
 bool tile_wanted(int batch, int n, int k) {
   if (umma_forced() >= 0) {
     return false;

@@ -1,14 +1,14 @@
 // Batches on the fifth-generation tensor cores, up to 128 rows a pass: one read of the weights
 // serves the whole batch, and the multiply-adds cost no issue slots.
 //
-// What bounds it. A tcgen05.mma kind::f16 of M = 128 takes ~45 clocks for every N up to 64 and
-// N / 2 clocks above; a step of 128 features x 256 output columns is 16 of them, 720 clocks up to
-// 64 rows against ~720 clocks of HBM time for its 17 KB of packets, and 1024 clocks at 128 rows,
-// where the tensor cores are the bound. The passes of 16 rows on mma.sync that this replaces pay
-// one whole read and unpack of the layer per 16 rows. Measured on 28672 x 8192, bf16, per call:
-// 51 / 57 / 68 / 108 / 204 us at 16 / 32 / 64 / 128 / 256 rows (58 / 112 / 221 / 437 / 862 in passes
-// of 16), i.e. ~2000 clocks a step up to 32 rows, where unpack -> MMA -> unpack is a chain through
-// two buffers per tile, and ~4200 at 128, where MMA -> promote -> MMA is one.
+// What bounds it: the hand-overs between its roles. A tcgen05.mma kind::f16 of M = 128 takes ~45 clocks
+// for every N up to 64; a step of 128 features x 256 output columns is 16 of them up to 64 rows, 720
+// clocks against ~770 clocks of HBM time for its 17 KB of packets, and 32 above (two halves of at most
+// 64 rows), 1440 clocks. A step takes ~2000 clocks up to 32 rows, where unpack -> MMA -> unpack is a chain
+// through two buffers per tile, ~2800 at 64 rows, and ~4200 at 128, where MMA -> promote -> MMA is one.
+// The passes of 16 rows on mma.sync that this replaces pay one whole read and unpack of the layer per
+// 16 rows. Measured on 28672 x 8192, bf16, per call: 51 / 57 / 68 / 108 / 204 us at 16 / 32 / 64 / 128 /
+// 256 rows (58 / 112 / 221 / 437 / 862 in passes of 16).
 //
 // Exactness. The unpacked operand is q - 8, exact in bf16 and in fp16, against the activations as
 // they are; every quantisation group has an accumulator of its own in tensor memory, and the
@@ -31,7 +31,8 @@
 //                          thread, two rows per packed FMA; stores finished columns
 // With 64 to 128 accumulators per thread the promote warps need more registers than an even split
 // of the file gives: instances of 64 and 128 rows move them there (2 x 184 + 2 x 40 + 24 = 472 per
-// lane position, of the 5 x 96 = 480 that the CTA is launched with).
+// lane position, of the 5 x 96 = 480 that the CTA is launched with). The 128-row instances, and those of
+// 64 rows for groups of 32 and 64, still spill 52 to 68 bytes a thread.
 #pragma once
 
 #include "w4a16_gemm_umma.cuh"

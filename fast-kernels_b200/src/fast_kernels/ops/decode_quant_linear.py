@@ -5,12 +5,13 @@ function names, keyword arguments, argument checks and error types (``TypeError`
 tensor type or dtype, ``ValueError`` for shapes, devices and option strings, ``RuntimeError`` when
 the native module is missing). What differs:
 
-* there is one implementation, the sm_100a kernel. The ``impl`` argument and the
+* the library picks its sm_100a kernel by the problem. The ``impl`` argument and the
   ``FK_ARC_W4A16_IMPL`` variable still accept ``auto | scalar | tc | wgmma`` (the reference's
-  tests pass them) but all of them run the same kernel; the cuBLASLt route stays available only
+  tests pass them) but all of them run the same; the cuBLASLt route stays available only
   as the baseline subject ``cublaslt_fp16_after_dequant``;
 * no autotuning and no separate group-sum launch: ``arc_w4a16_forward`` is a single kernel launch
-  that also finishes split-K; ``split_k_slices > 1`` selects the caller-visible partials path;
+  that also finishes split-K, with a small one ahead of it that lays out the activations where the
+  batch runs on the tensor cores; ``split_k_slices > 1`` selects the caller-visible partials path;
 * ``torch.bfloat16`` tensors and ``group_size=32`` are accepted everywhere (the 16-bit dtype of
   activations, scales, offsets and outputs must agree).
 

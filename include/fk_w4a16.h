@@ -74,10 +74,11 @@ FK_W4A16_API int fk_w4a16_group_sums(const void* activations, float* sums, int b
 FK_W4A16_API size_t fk_w4a16_workspace_bytes(int batch, int n, int k, int group_size);
 FK_W4A16_API int fk_w4a16_workspace_init(void* workspace, size_t workspace_bytes, void* stream);
 
-/* The hot path: out[batch, n] = activations[batch, k] . W^T in ONE launch -- activation group
- * sums, int4 unpack, scale/offset, fp32 accumulation, split-K finish and the 16-bit rounding of
- * the output all happen inside it. batch <= 4 streams on CUDA cores; larger batches are
- * processed 4 rows at a time.
+/* The hot path: out[batch, n] = activations[batch, k] . W^T -- activation group sums, int4 unpack,
+ * scale/offset, fp32 accumulation, split-K finish and the 16-bit rounding of the output in one
+ * call. batch <= 4 streams on CUDA cores in ONE launch (batches 2 to 4 of large layers take the next
+ * kernel); up to 8 rows run on mma.sync behind a small launch that lays out the activations, larger
+ * batches on tcgen05 in passes of up to 128 rows, likewise (fk_w4a16_set_variant, below, says where not).
  * Reference: arc_w4a16_forward, arc_w4a16.cu:687-707, together with the group-sum prepass
  * (:671-685) and the split-K pair (:709-751) that its Python caller chains around it
  * (src/fast_kernels/ops/decode_quant_linear.py:383-439). */
@@ -288,34 +289,40 @@ FK_W4A16_API int fk_w4a16_cublaslt_matmul(const void* activations, const void* w
 FK_W4A16_API int fk_w4a16_device_status(int* status);
 
 /* Launch-shape knobs of the fused GEMV, for tuning and tests: warps per CTA (1..16, 0 = auto),
- * ring stages per warp (1..8, 0 = auto) and CTAs in the grid (0 = one per SM). Process-wide. */
+ * ring stages per warp (1..8, 0 = auto) and CTAs in the grid (0 = one per SM). Process-wide. A warp
+ * count keeps every batch on the kernels that have one (the tcgen05 kernels do not). */
 FK_W4A16_API int fk_w4a16_set_launch_config(int warps_per_cta, int stages, int ctas);
 
 /* Writes a one-line description of the launch fk_w4a16_gemv would make for a problem on the current
- * device -- kernel name with its template arguments, grid, cluster size, warps, ring stages,
- * shared memory -- into text[capacity] (host pointer). For benchmarks and profiles that attribute
- * time to kernels; no counterpart in the reference. */
+ * device -- kernel name with its template arguments, grid, cluster size, warps, ring stages, shared
+ * memory, and for the tile kernel the rows of a pass and the passes -- into text[capacity] (host
+ * pointer; 128 characters hold it). For benchmarks and profiles that attribute time to kernels; no
+ * counterpart in the reference. */
 FK_W4A16_API int fk_w4a16_describe_plan(int batch, int n, int k, int group_size, int dtype, char* text,
                            size_t capacity);
 
 /* Launch-plan thresholds, process-wide, for tuning and tests (no counterpart in the reference).
  * Each knob starts from an environment variable that is read once, at the library's first
  * planning call: "mma_min_batch" (FK_W4A16_MMA_MIN_BATCH: smallest batch that takes the mma.sync
- * kernel, 0 = built-in rule), "cluster_min" / "cluster_size" (FK_W4A16_CLUSTER_MIN / _SIZE),
+ * kernel, 0 = built-in rule; set, it holds for every batch, unless "tile_min_batch" is set too),
+ * "cluster_min" / "cluster_size" (FK_W4A16_CLUSTER_MIN / _SIZE),
  * "wmma" (FK_W4A16_WMMA: batches 1-2 on the warp-level mma.sync form of the stream kernel),
  * "cluster" (FK_W4A16_CLUSTER: 0 keeps every layer off the cluster kernel),
  * "umma_min_batch" (FK_W4A16_UMMA_MIN_BATCH: smallest batch that takes the pipelined tcgen05
- * kernel, 0 = never, -1 = built-in default), "peer_wait_ms" (FK_W4A16_PEER_WAIT_MS: how long a
- * multi-GPU call waits for the other GPUs before it gives up, default 2000). Results never depend
- * on them beyond the order of fp32 additions. */
+ * kernel, 0 = never, -1 = built-in default), "tile_min_batch" (FK_W4A16_TILE_MIN_BATCH: smallest batch
+ * that takes the tcgen05 tile kernel, 0 = never, -1 = built-in rule), "peer_wait_ms"
+ * (FK_W4A16_PEER_WAIT_MS: how long a multi-GPU call waits for the other GPUs before it gives up,
+ * default 2000). Results never depend on them beyond the rounding of fp32 sums. */
 FK_W4A16_API int fk_w4a16_set_tuning(const char* name, int value);
 
 /* Kernel variant of the fused GEMV, process-wide, for measurements and tests (no counterpart in
- * the reference). AUTO picks per problem between the CUDA-core stream kernel, its cluster form and
- * the mma.sync kernel; TCGEN05 forces the warp-specialised tcgen05 / tensor-memory kernel for every
- * batch size -- same results, slower on decode shapes (its header says why); CLASSIC never uses
- * it. The environment variable FK_W4A16_TC5=1 selects TCGEN05 when this function was never
- * called. */
+ * the reference). AUTO picks per problem between the CUDA-core stream kernel, its cluster form, the
+ * mma.sync kernel and, above 8 rows, the tcgen05 tile kernel (above 64 rows on layers of at least
+ * 6 * 2^20 weights; not for gated or multi-GPU calls, nor where the workspace holds the mma.sync
+ * plan only). TCGEN05 forces the warp-specialised tcgen05 / tensor-memory pipeline for every
+ * batch size -- same results, slower on decode shapes (its header says why); CLASSIC uses neither of
+ * the two tcgen05 kernels. The environment variable FK_W4A16_TC5=1 selects TCGEN05 when this
+ * function was never called. */
 #define FK_W4A16_VARIANT_AUTO 0
 #define FK_W4A16_VARIANT_TCGEN05 1
 #define FK_W4A16_VARIANT_CLASSIC 2
