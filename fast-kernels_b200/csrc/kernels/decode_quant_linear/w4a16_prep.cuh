@@ -94,8 +94,10 @@ __global__ void __launch_bounds__(256) dequant_rowmajor_kernel(const uint8_t* __
 // byte in), which therefore go out as whole rows of the group, G * 2 contiguous bytes, 16 per
 // thread. (Stored straight from the packet's column order, every 16 bytes went to another row: half
 // a sector each; 28672 x 4096, groups of 128: 155 us, now 55.7, of which the bytes need 45 at the
-// measured HBM rate; groups of 64 / 32: 154 / 149, now 61.5 / 64.3.) The pitch lets the G / 8 words of the rows of a warp be read without conflicts.
-// The packets are only known to be 4-byte aligned, hence 32-bit loads.
+// measured HBM rate; groups of 64 / 32: 154 / 149, now 61.5 / 64.3. Below 64 packets its few blocks take
+// 0.5 to 0.9 us longer than that: 512 x 1024, 2.7 against 2.0; blocks of 1024 threads took 3.0.) The pitch
+// lets the G / 8 words of the rows of a warp be read without conflicts. The packets are only known to be
+// 4-byte aligned, hence 32-bit loads.
 template <int G, class E>
 __global__ void __launch_bounds__(256) dequant_packets_kernel(const uint8_t* __restrict__ packets,
                                                               uint16_t* __restrict__ out,

@@ -102,6 +102,30 @@ def test_pack_and_dequant_are_bit_exact(group: int, dtype: str) -> None:
 
 @pytest.mark.parametrize("group", [32, 64, 128])
 @pytest.mark.parametrize("dtype", ["fp16", "bf16"])
+@pytest.mark.parametrize(("tiles", "groups"), [
+    (1, 1), (149, 1),
+    (41, 29),                   # more than the 8 blocks of every SM: some expand a second packet
+])
+def test_pack_and_dequant_of_few_and_many_packets(group: int, dtype: str, tiles: int, groups: int) -> None:
+    code = oracle.dtype_code(dtype)
+    shape = LayerShape("t", 128 * tiles, group * groups, group_size=group, dtype=dtype, zero_point=None,
+                       scale_range=(0.001, 0.05))
+    problem = make_problem(shape, seed=tiles + group)
+    q, alpha, beta = (problem[k].cuda() for k in ("q_u8", "alpha", "beta"))
+    packets = capi_pack(capi, q, alpha, beta, group)
+    assert np.array_equal(packets.cpu().numpy(),
+                          oracle.pack_packets(problem["q_u8"].numpy(), oracle.bits_of(problem["alpha"]),
+                                              oracle.bits_of(problem["beta"]), group))
+    weight = torch.zeros((shape.n, shape.k), dtype=alpha.dtype, device="cuda")
+    capi.check(capi.load_library().fk_w4a16_dequant_packets(packets.data_ptr(), weight.data_ptr(), shape.n, shape.k,
+                                                            group, capi.packet_stride_bytes(group), code, stream_ptr()))
+    assert np.array_equal(host_bits(weight),
+                          oracle.dequant_rowmajor(problem["q_u8"].numpy(), oracle.bits_of(problem["alpha"]),
+                                                  oracle.bits_of(problem["beta"]), group, code))
+
+
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize("dtype", ["fp16", "bf16"])
 def test_group_sums_are_bit_exact(group: int, dtype: str) -> None:
     code = oracle.dtype_code(dtype)
     gen = torch.Generator().manual_seed(5 + group)
